@@ -244,6 +244,7 @@ struct tpm_ctx {
   // largest exponent fields of U and RU_int at each stage (k_face_velocity_max:
   // 2 x 4), of P and the face coefficients in a solve (k_fx_maxima: 2)
   unsigned *fx_emax = nullptr;
+  bool fx_emax_stale = false;  // RU_int has been uploaded since the stage's face velocity
   const double2 *r2c64 = nullptr;
   const float2 *r2c32 = nullptr;
   double *err_parts = nullptr;  // one max|dp| per x-pass block (sized for one row per block)
