@@ -114,3 +114,30 @@ def test_pcg_graph_bit_identical_and_mixed_close(capi):
     mixed = run(capi, p2.replace(precision=P.PREC_MIXED), s, 3)
     for f in ("RU", "RHO", "P"):
         assert rel_err(mixed.download_field(f), eager.download_field(f)) <= 1e-5, f
+
+
+def test_heated_pcg_box_does_not_depend_on_batch_or_tiles(capi):
+    """A heated FP64 box solved by conjugate gradients gives the same bits alone,
+    in a batch and with other transform tiles: r.z is summed by groups of rows
+    that only the grid decides."""
+    from test_gpu_graph import assert_same, state
+
+    p, s = case(2)
+    want = state(run(capi, p, s, 2))
+    b = capi.Batch([p, p], [s.npart, s.npart])
+    for box in b.boxes:
+        box.load(s)
+        box.initialize()
+    b.run(2)
+    b.sync()
+    got = [state(box) for box in b.boxes]
+    b.close()
+    for tiles in ([1, 2, 4, 64, 96, 160], [8, 4, 8, 128, 64, 128]):
+        ctx = capi.Context(p, s.npart)
+        ctx.load(s)
+        ctx.set_fft_tiles(tiles)
+        ctx.initialize()
+        ctx.run(2)
+        got.append(state(ctx))
+    for g in got:
+        assert_same(g, want)
