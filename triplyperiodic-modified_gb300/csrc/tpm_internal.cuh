@@ -242,7 +242,8 @@ struct tpm_ctx {
   long long *fx_inv = nullptr;  // per mode: 1/(ax + ay + az), scaled per (kx, ky) pencil
   int *fx_inv_e = nullptr;      // that scale's exponent
   // largest exponent fields of U and RU_int at each stage (k_face_velocity_max:
-  // 2 x 4), of P and the face coefficients in a solve (k_fx_maxima: 2)
+  // 2 x 4), of P and the face coefficients in a solve (k_fx_maxima: 2), of the P
+  // that an iteration writes
   unsigned *fx_emax = nullptr;
   bool fx_emax_stale = false;  // RU_int has been uploaded since the stage's face velocity
   const double2 *r2c64 = nullptr;
