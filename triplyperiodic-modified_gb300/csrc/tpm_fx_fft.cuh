@@ -383,11 +383,17 @@ k_fx_xfwd(Grid g, FxPlan pl, const FxTw *__restrict__ r2c, Src src, double2 *__r
     int j = 0, k = 0;
     if (in) row_jk(g, row, j, k);
     src.row(g, j, k);
-    for (; m < count; m += step) {
-      const double2 r = in ? src(g, m) : make_double2(0, 0);
-      out[m] = r;
-      e = max(e, max(fx_exp(r.x), fx_exp(r.y)));
-    }
+    auto cells = [&](auto &&pair) {
+      for (; m < count; m += step) {
+        const double2 r = in ? pair(m) : make_double2(0, 0);
+        out[m] = r;
+        e = max(e, max(fx_exp(r.x), fx_exp(r.y)));
+      }
+    };
+    if (src.wide)  // (the same for all rows)
+      cells([&](int i) { return src.fp64_pair(g, i); });
+    else
+      cells([&](int i) { return src(g, i); });
     e = __reduce_max_sync(0xffffffffu, e);
     if ((threadIdx.x & 31) == 0) atomicMax(&sc.emax[q], e);
   });
