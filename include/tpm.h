@@ -48,7 +48,19 @@ enum {
 
 /* ---- arithmetic of the substep ---- */
 enum {
-  TPM_PREC_FP64 = 0,  /* plain FP64 path, parity with the reference */
+  TPM_PREC_FP64 = 0,  /* parity with the reference (1e-12 per field and step).
+                         Unheated boxes (I01 = I02 = 0): FP64 throughout.
+                         Heated ones: transforms, residuals, momentum terms and
+                         particle deposits in 64-bit integers scaled to the
+                         largest value of the field (a transform: of the pencil;
+                         a deposit: of all particles' rates), which is closer to
+                         the exact result in the norm of the field, but what a
+                         value far below the largest keeps is an absolute
+                         accuracy: momentum terms round at some 2^-56 of the
+                         field's largest, deposits at 2^-62 of the largest rate
+                         (2^-61 of a particle for the concentration).  Face
+                         coefficients whose range exceeds 2^8 take the FP64
+                         residual. */
   TPM_PREC_MIXED = 1  /* FP32 stencils/FFT/particles, FP64 state, means and
                          one FP64 defect-correction projection */
 };
