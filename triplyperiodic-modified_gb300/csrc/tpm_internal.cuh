@@ -248,7 +248,6 @@ struct tpm_ctx {
   bool fx_emax_stale = false;  // RU_int has been uploaded since the stage's face velocity
   const double2 *r2c64 = nullptr;
   const float2 *r2c32 = nullptr;
-  double *err_parts = nullptr;  // one max|dp| per x-pass block (sized for one row per block)
   int pen[3] = {1, 1, 1};       // FFT pencils per block of the x, y, z passes (autotuned)
   int fthreads[3] = {256, 256, 256};  // threads per block of the x, y, z passes (autotuned)
   bool device_loop = false;     // Poisson stopping test on the device (no host read)
