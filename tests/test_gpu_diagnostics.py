@@ -183,6 +183,29 @@ def test_rdf_pairs_at_bin_edges(capi, oracle_lib, share):
     assert np.array_equal(pairs, want)
 
 
+@pytest.mark.parametrize("units", [2.0 / 3.0, 0.4, 1.0])
+def test_rdf_pairs_of_bins_finer_than_the_integer_positions(capi, oracle_lib, units):
+    """Bins of about 2^-32 of the box, finer than single precision and integer
+    positions tell apart: every pair is binned in FP64, those half a bin from the
+    edges too."""
+    p, s = case(N=24, npart=4000, seed=13)
+    p = p.replace(Lx=1.0, Ly=1.0, Lz=1.0)
+    rng = np.random.default_rng(13)
+    for q in ("x", "y", "z"):
+        s.part[q] = np.repeat(0.1 + 0.8 * rng.random(s.npart // 20), 20)
+    s.part["x"] += 8 * 2.0 ** -32 * rng.random(s.npart)
+    nb = 12
+    r_max = nb * units * 2.0 ** -32
+    ctx = capi.Context(p, s.npart)
+    ctx.load(s)
+    ctx.initialize()
+    base = ctx.download_particles("base")
+    pairs, _ = ctx.rdf(r_max, nb)
+    want = oracle_lib.rdf_pairs(base["x"], base["y"], base["z"], (1.0, 1.0, 1.0), r_max, nb)
+    assert want.sum() > 1000
+    assert np.array_equal(pairs, want)
+
+
 def test_rdf_rejects_r_max_beyond_a_third_of_the_box(capi):
     p, s = case(N=16, npart=100)
     ctx = capi.Context(p, s.npart)

@@ -342,7 +342,7 @@ k_rdf_pairs(RdfGrid r, RdfPairs q, int64_t np, const double *__restrict__ pos,
             const float t = sqrtf(r2) * q.inv_dr;
             int bin = (int)t;
             const float f = t - (float)bin;
-            if (f < q.eps || f > 1.f - q.eps) bin = rdf_bin(r, q, pos, np, b, xa, ya, za);
+            if (f <= q.eps || f >= 1.f - q.eps) bin = rdf_bin(r, q, pos, np, b, xa, ya, za);
             count(bin);
           }
         }
