@@ -278,3 +278,20 @@ def test_adjoint_64_over_the_200_step_horizon(capi):
     assert np.all(np.isfinite(g1)) and np.isfinite(gA1) and np.isfinite(gt1)
     assert rel_err(g2, g1) <= 1e-13
     assert abs(gA2 - gA1) <= 1e-13 * abs(gA1) and abs(gt2 - gt1) <= 1e-13 * abs(gt1)
+
+
+def test_unheated_context_makes_the_adjoints_tables_with_the_first_adjoint(capi):
+    """An unheated FP64 context holds the FP64 passes' table and not the fixed-point
+    ones too (8.5 MB each at 128^3), which only the adjoint's projections read: it
+    takes no more memory than a heated one, whose steps read those instead."""
+    import torch
+
+    p = P.physical(128, 10, nu=0.03, A=0.1, tau_p=0.1, mass_loading=0.3, heating_Q=0.5)
+    used = {}
+    capi.Context(p, 10).close()  # (the process's first context loads the kernels)
+    for name, q in (("heated", p), ("unheated", p.replace(I01=0.0, I02=0.0))):
+        before = torch.cuda.mem_get_info()[0]
+        ctx = capi.Context(q, 10)
+        used[name] = before - torch.cuda.mem_get_info()[0]
+        ctx.close()
+    assert used["unheated"] <= used["heated"] + (4 << 20)

@@ -688,6 +688,7 @@ extern "C" int tpm_adjoint_run(tpm_ctx *c, int nsteps, int checkpoint_every, dou
       TPM_CUDA_TRY(cudaMemcpy(A.ones, ones.data(), sizeof(double) * A.n, cudaMemcpyHostToDevice));
     }
     precondition_setup();
+    fx_plans_create(c);
     TPM_CUDA_TRY(cudaMemsetAsync(A.gscal, 0, sizeof(double) * 4, c->stream));
     const bool prof = c->prof_on;
     c->prof_on = false;

@@ -399,6 +399,7 @@ void launch_to_double(tpm_ctx *c, const float *src, double *dst, long long n);
 
 // ---- Poisson / FFT (tpm_fft.cu) ----
 void fft_plans_create(tpm_ctx *c);
+void fx_plans_create(tpm_ctx *c);  // the fixed-point passes' (before fft_precondition's fx)
 // A Richardson loop captured as a conditional while node: the body's last
 // kernel sets `handle` to continue while it < max_it and max|dp| > epsilon.
 struct LoopCtl {
