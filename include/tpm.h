@@ -421,14 +421,17 @@ int tpm_adjoint_run(tpm_ctx *ctx, int nsteps, int checkpoint_every, double w_tke
  * context's grid; results do not depend on the choice (each pencil is
  * transformed independently).  The state is kept: P and the device scalars
  * are restored afterwards.  pens_out (6 ints, optional) receives the pencils
- * of the x, y, z passes, then their threads per block. */
+ * of the x, y, z passes, then their threads per block.  The fixed-point passes
+ * of heated FP64 boxes (pencils of at most 256 points) take at most 32 pencils
+ * and as many threads as follow from them: there the threads are not searched
+ * and not used. */
 int tpm_autotune(tpm_ctx *ctx, int *pens_out);
 
 /* Sets the FFT tiles that tpm_autotune would pick, e.g. ones it picked before
  * for the same grid: tiles[0..2] the pencils per block of the x, y, z passes
  * (powers of two, at most what the passes' shared memory holds), tiles[3..5]
- * their threads per block (multiples of 32, 32..1024).  Results do not depend
- * on the tiles.  TPM_ERR_ARG for values out of range.  Not in the reference. */
+ * their threads per block (multiples of 32, 32..1024; see tpm_autotune for the
+ * passes that do not use them).  Results do not depend on the tiles.  TPM_ERR_ARG for values out of range.  Not in the reference. */
 int tpm_set_fft_tiles(tpm_ctx *ctx, const int *tiles);
 
 /* ---------------------------------------------------------------- ensembles

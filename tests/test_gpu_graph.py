@@ -211,3 +211,18 @@ def test_step_state_equals_load_step_save(capi, prec, graph, npart):
     c.step()
     for f in ("RU", "RHO", "P", "C", "Q"):
         assert np.array_equal(b.download_field(f), c.download_field(f)), f
+
+
+def test_autotune_of_fixed_point_passes_times_each_tile_once(capi):
+    """The fixed-point passes of a heated FP64 box take their threads from their
+    pencils, at most 32: the search times at most six tiles per pass (four
+    iterations of five launches and the solve's scales each) and leaves the
+    threads alone."""
+    p, s = case(dims=(24, 24, 24), npart=100)
+    ctx = capi.Context(p, s.npart)
+    ctx.load(s)
+    ctx.initialize()
+    before = ctx.launch_count()
+    tiles = ctx.autotune()
+    assert ctx.launch_count() - before <= 3 * 6 * (4 * 5 + 1)
+    assert ctx.autotune()[3:] == tiles[3:]

@@ -245,7 +245,9 @@ void graphs_clear(std::vector<GraphEntry> &cache) {
 }
 
 // Coordinate search over the pencils per block, then the threads per block,
-// of the x, y and z passes.
+// of the x, y and z passes.  The fixed-point passes take their threads from
+// their pencils, and of these no more than they have use for: what would launch
+// the same again is not timed.
 void autotune(tpm_ctx *c) {
   const Grid &g = c->g;
   const int n_of[3] = {c->fx.n, c->fy.n, c->fz.n};
@@ -276,10 +278,18 @@ void autotune(tpm_ctx *c) {
     const int cap = pens_max(n_of[d], c->p.precision == TPM_PREC_MIXED ? 8 : 16);
     int best = c->pen[d];
     double best_ms = time_iterations(c, e0, e1, reps);
+    const int fx = fx_pass_pens(c, d);  // 0: not a fixed-point pass
+    unsigned timed = fx;                // (powers of two: a bit each)
     for (int cand = 1; cand <= cap; cand *= 2) {
       if (cand == best) continue;
       const int keep = c->pen[d];
       c->pen[d] = cand;
+      const unsigned same = timed & fx_pass_pens(c, d);
+      timed |= fx_pass_pens(c, d);
+      if (same) {
+        c->pen[d] = keep;
+        continue;
+      }
       const double ms = time_iterations(c, e0, e1, reps);
       if (ms < 0.97 * best_ms) {  // keep the incumbent unless clearly faster
         best_ms = ms;
@@ -290,7 +300,7 @@ void autotune(tpm_ctx *c) {
     c->pen[d] = best;
     int best_t = c->fthreads[d];
     for (int th : {128, 256, 512}) {
-      if (th == best_t) continue;
+      if (th == best_t || fx) continue;
       const int keep = c->fthreads[d];
       c->fthreads[d] = th;
       const double ms = time_iterations(c, e0, e1, reps);

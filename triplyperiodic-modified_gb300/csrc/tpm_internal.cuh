@@ -417,6 +417,9 @@ void poisson_iteration(tpm_ctx *c, double eps_ctl = -1.0, const LoopCtl *loop = 
 void poisson_loop_begin(tpm_ctx *c);
 // FP64 path, heated: the scales of a solve's fixed-point residual
 void fx_solve_begin(tpm_ctx *c);
+// pencils per block of the Richardson iteration's pass d (x, y, z) with the present
+// tiles where it is a fixed-point one, else 0
+int fx_pass_pens(const tpm_ctx *c, int d);
 // the transform passes' tiles, for a box that runs beside boxes - 1 others
 void default_tiles(tpm_ctx *c, int boxes);
 // mixed Richardson loop: P += dP after the loop (a no-op below two iterations);
