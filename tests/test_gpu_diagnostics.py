@@ -206,6 +206,24 @@ def test_rdf_pairs_of_bins_finer_than_the_integer_positions(capi, oracle_lib, un
     assert np.array_equal(pairs, want)
 
 
+@pytest.mark.parametrize("L", [3e-20, 1.0, 1e20])
+def test_rdf_pairs_in_any_unit_of_length(capi, oracle_lib, L):
+    """The single-precision form of the pairs counts in bins: a box whose squared
+    lengths leave the range of single precision gets the same counts."""
+    p, s = case(N=24, npart=3000, seed=14)
+    rng = np.random.default_rng(14)
+    for q in ("x", "y", "z"):
+        s.part[q] = L * rng.random(s.npart)
+    p = p.replace(Lx=L, Ly=L, Lz=L)
+    ctx = capi.Context(p, s.npart)
+    ctx.load(s)
+    ctx.initialize()
+    base = ctx.download_particles("base")
+    pairs, _ = ctx.rdf(L / 3, 32)
+    want = oracle_lib.rdf_pairs(base["x"], base["y"], base["z"], (L, L, L), L / 3, 32)
+    assert np.array_equal(pairs, want)
+
+
 def test_rdf_rejects_r_max_beyond_a_third_of_the_box(capi):
     p, s = case(N=16, npart=100)
     ctx = capi.Context(p, s.npart)

@@ -286,8 +286,9 @@ __device__ __forceinline__ double min_image(double d, double L, double h) {
 // in FP64.  The counts are the FP64 form's, bit for bit.
 struct RdfPairs {
   double r_max2, dr;
-  float sx, sy, sz;  // box lengths times 2^-32
-  float inv_dr, eps, far2;  // far2: r^2 past the last bin and eps
+  // in bins, whatever the box's unit of length: box lengths times 2^-32, the error
+  // of r and (squared) what lies past the last bin and that
+  float sx, sy, sz, eps, far2;
   int nbins, copies;  // copies of the histogram in shared memory
 };
 __device__ __forceinline__ int rdf_bin(const RdfGrid &r, const RdfPairs &q,
@@ -339,7 +340,7 @@ k_rdf_pairs(RdfGrid r, RdfPairs q, int64_t np, const double *__restrict__ pos,
             const float fz = (float)(int)((unsigned)ib.z - (unsigned)ia.z) * q.sz;
             const float r2 = fmaf(fx, fx, fmaf(fy, fy, fz * fz));
             if (r2 > q.far2) continue;
-            const float t = sqrtf(r2) * q.inv_dr;
+            const float t = sqrtf(r2);
             int bin = (int)t;
             const float f = t - (float)bin;
             if (f <= q.eps || f >= 1.f - q.eps) bin = rdf_bin(r, q, pos, np, b, xa, ya, za);
@@ -581,15 +582,14 @@ int tpm_rdf(tpm_ctx *c, double r_max, int nbins, unsigned long long *pairs, doub
       q.r_max2 = r_max * r_max;
       q.dr = r_max / nbins;
       const double two32 = 1.0 / 4294967296.0, Lm = std::max(L[0], std::max(L[1], L[2]));
-      q.sx = (float)(L[0] * two32);
-      q.sy = (float)(L[1] * two32);
-      q.sz = (float)(L[2] * two32);
-      q.inv_dr = (float)(1.0 / q.dr);
+      q.sx = (float)(L[0] * two32 / q.dr);
+      q.sy = (float)(L[1] * two32 / q.dr);
+      q.sz = (float)(L[2] * two32 / q.dr);
       // error of r / dr: two truncations of 2^-32 L per direction, and the FP32
-      // roundings (a conversion, two products, the sum, the root: 2^-21 of it)
+      // roundings (two conversions, a product, the sum, the root: 2^-21 of it)
       const double eps = 4 * Lm * two32 / q.dr + nbins * 0x1p-20;
       q.eps = (float)(eps < 0.5 ? eps : 0.5);  // (0.5: every candidate in FP64)
-      q.far2 = (float)(q.r_max2 * std::pow(1 + 2 * eps / nbins, 2));
+      q.far2 = (float)std::pow(nbins + 2 * eps, 2);
       q.nbins = nbins;
       q.copies = nbins <= 512 ? kDiagThreads / 32 : 1;
       const int qb = (int)((c->np + kDiagThreads - 1) / kDiagThreads);
