@@ -59,7 +59,7 @@ enum {
                          accuracy: momentum terms round at some 2^-56 of the
                          field's largest, deposits at 2^-62 of the largest rate
                          (2^-61 of a particle for the concentration).  Face
-                         coefficients whose range exceeds 2^8 take the FP64
+                         coefficients whose range exceeds 2^9 take the FP64
                          residual. */
   TPM_PREC_MIXED = 1  /* FP32 stencils/FFT/particles, FP64 state, means and
                          one FP64 defect-correction projection */
