@@ -355,9 +355,8 @@ __global__ void k_adj_particles(Grid g, int64_t np, PAdj s, const double *__rest
 // ------------------------------------------------------------------ gas RHS
 // U = RU / Rho_face of a recorded stage.  The transposed stencil below reads
 // each face's velocity from up to 12 cells; formed there, its 36 divisions per
-// cell were most of the stencil's FP64 work (64^3, 2e5 particles, 20 steps:
-// 191 ms before, 140 with this, the wraps by comparison and the last segment
-// recorded on the way).
+// cell were most of the stencil's FP64 work (64^3, 2e5 particles, 20 steps: 137 ms;
+// 191 without this, the wraps by comparison and the last segment recorded on the way).
 __global__ void k_adj_velocity(Grid g, const double *__restrict__ RU,
                                const double *__restrict__ Rho, double *__restrict__ U) {
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.n;

@@ -188,7 +188,7 @@ __device__ __forceinline__ int fx_scale_of(const FxScales &sc, int q, int more) 
 }
 
 // ------------------------------------------------------------------ y passes
-// (five blocks per SM: 128^3 22.8 us against 29.3 with four; 256^3 116 to 113)
+// (five blocks per SM: 128^3 22.8 us, with four 29.3; 256^3 116 us, with four 3 % more)
 template <int SIGN>
 __global__ void __launch_bounds__(kFxItems, 5)
 k_fx_y(Grid g, FxPlan pl, double2 *__restrict__ spec, int lq, const int *__restrict__ skip) {
@@ -366,7 +366,7 @@ __device__ __forceinline__ fx2 *fx_row_transform(const FxPlan &pl, int lq, FxSca
 
 // The x passes run three blocks of 256 threads per SM (at most 85 registers):
 // with two, 16 warps left the waits for rows and barriers uncovered (256^3,
-// inverse: 314 -> 267 us, by pairs of cells 245; a fourth block spills, 285).
+// inverse: 244 us; single cells 267, with two blocks 314; a fourth block spills, 285).
 //
 // forward x pass of the rows src(g, m), the cells 2 m and 2 m + 1 of row (j, k):
 // real-to-complex
