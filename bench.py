@@ -701,7 +701,9 @@ def gpu_main(args):
 
     cmp = {}
     for name, r_ in res.items():
-        per_it = sum(r_["kernels_ms_per_step"].get(k, 0.0) for k in FFT_KERNELS) / (4 * r_["n_it"])
+        # (the profiled steps' own iterations, which the timed steps' mean need not be)
+        per_it = (sum(r_["kernels_ms_per_step"].get(k, 0.0) for k in FFT_KERNELS)
+                  / r_["kernel_launches_per_step"]["fft_x_fwd_resid"])
         dtype = torch.float32 if name == "mixed" else torch.float64
         cmp[name] = {"own_iteration_ms": round(per_it, 4),
                      "cufft_solve_ms": round(cufft_solve_ms((p64.Nz, p64.Ny, p64.Nx),
