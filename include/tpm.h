@@ -424,7 +424,8 @@ int tpm_adjoint_run(tpm_ctx *ctx, int nsteps, int checkpoint_every, double w_tke
  * of the x, y, z passes, then their threads per block.  The fixed-point passes
  * of heated FP64 boxes (pencils of at most 256 points) take at most 32 pencils
  * and as many threads as follow from them: there the threads are not searched
- * and not used. */
+ * and not used.  The x passes of a PCG solve (Solver = 2), which sum r.z by their
+ * blocks, use neither. */
 int tpm_autotune(tpm_ctx *ctx, int *pens_out);
 
 /* Sets the FFT tiles that tpm_autotune would pick, e.g. ones it picked before

@@ -141,3 +141,21 @@ def test_heated_pcg_box_does_not_depend_on_batch_or_tiles(capi):
         got.append(state(ctx))
     for g in got:
         assert_same(g, want)
+
+
+@pytest.mark.parametrize("heat,prec", [(0.0, P.PREC_FP64), (0.5, P.PREC_MIXED)])
+def test_pcg_box_does_not_depend_on_tiles(capi, heat, prec):
+    """The same of the FP64 and the mixed passes: tiles that an autotuner might pick
+    leave every bit of a conjugate-gradient solve alone."""
+    from test_gpu_graph import assert_same, state
+
+    p, s = case(2, prec)
+    p = p.replace(I01=heat * p.I01, I02=heat * p.I02)
+    want = state(run(capi, p, s, 2))
+    for tiles in ([1, 2, 4, 64, 96, 160], [8, 4, 8, 128, 64, 128]):
+        ctx = capi.Context(p, s.npart)
+        ctx.load(s)
+        ctx.set_fft_tiles(tiles)
+        ctx.initialize()
+        ctx.run(2)
+        assert_same(state(ctx), want)
